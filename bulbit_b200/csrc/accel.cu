@@ -121,9 +121,9 @@ struct BatchSrc
 // Ordered traversal: persistent warps pulling rays from a work counter, over
 // the child-box layout or (WIDE) the 8-wide layout.
 template <bool ANY, bool WIDE, bool SPHERES = true>
-__global__ void __launch_bounds__(kTraceBlock) PersistentTraceKernel(AccelView a, const float4* __restrict__ rays,
-                                                                     int32_t n, float4* __restrict__ hits,
-                                                                     uint8_t* __restrict__ occluded, int32_t* next)
+__global__ void __launch_bounds__(kTraceBlock, TraceMinBlocks(kTraceBlock, WIDE))
+    PersistentTraceKernel(AccelView a, const float4* __restrict__ rays, int32_t n, float4* __restrict__ hits,
+                          uint8_t* __restrict__ occluded, int32_t* next)
 {
     BatchSrc<ANY> src{ rays, hits, occluded };
     if constexpr (WIDE)

@@ -53,8 +53,8 @@ struct StaticSrc
 };
 
 template <bool WIDE>
-__global__ void __launch_bounds__(kBlock) StaticTraceKernel(AccelView a, const float4* rays, int32_t n, float4* hits,
-                                                            int32_t* next)
+__global__ void __launch_bounds__(kBlock, TraceMinBlocks(kBlock, WIDE))
+    StaticTraceKernel(AccelView a, const float4* rays, int32_t n, float4* hits, int32_t* next)
 {
     StaticSrc src{ rays, hits };
     if constexpr (WIDE)

@@ -426,7 +426,7 @@ constexpr int kNumShapes = 4;
 constexpr TraversalShape kShapes[kNumShapes] = { { 128, 16 }, { 128, 0 }, { 128, 8 }, { 256, 16 } };
 
 template <class Scenes, int BLOCK = kBlock, int SHORT = kShortStack, bool WIDE = false, bool SPHERES = true>
-__global__ void __launch_bounds__(BLOCK) ClosestKernel(Scenes sc, WaveDev w, int parity)
+__global__ void __launch_bounds__(BLOCK, TraceMinBlocks(BLOCK, WIDE)) ClosestKernel(Scenes sc, WaveDev w, int parity)
 {
     const int32_t n = w.counts[parity];
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(BLOCK) ClosestKernel(Scenes sc, WaveDev w, int
 }
 
 template <class Scenes, int BLOCK = kBlock, int SHORT = kShortStack, bool WIDE = false, bool SPHERES = true>
-__global__ void __launch_bounds__(BLOCK) ShadowKernel(Scenes sc, WaveDev w)
+__global__ void __launch_bounds__(BLOCK, TraceMinBlocks(BLOCK, WIDE)) ShadowKernel(Scenes sc, WaveDev w)
 {
     const int32_t n = w.counts[2];
     if (blockIdx.x == 0 && threadIdx.x == 0)
