@@ -57,7 +57,8 @@ constexpr int kCBias = kCB3 + kGuideOut; // 232
 // a layer of N outputs (NT = N/8 tiles) and K inputs, element
 // ((kt * NT + nt) * 32 + lane) * 4 + e holds W[n][k] with n = nt*8 + lane/4
 // and k = kt*16 + 2*(lane%4) + {0, 1, 8, 9}[e]. The transposed images
-// (kBfT1..kBfT3, backward pass) are row-major.
+// (kBfT1..kBfT3, backward pass) are in fragment order too, with W^T[n][k] =
+// W[k][n] (row-major they cost eight bank conflicts a load).
 constexpr int kBf0 = 0;
 constexpr int kBf1 = kBf0 + kGuideHidden * kGuideIn;
 constexpr int kBf2 = kBf1 + kGuideHidden * kGuideHidden;
@@ -161,18 +162,8 @@ __device__ __forceinline__ void Mma16816(float* d, const uint32_t* a, uint32_t b
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// B fragment of an m16n8k16 MMA from a matrix stored [n][k] (k contiguous),
-// row stride ld elements: (k = 2t, 2t+1 | 2t+8, 2t+9; n = g).
-__device__ __forceinline__ void LoadB(const __nv_bfloat16* w, int ld, int n0, int k0, int lane, uint32_t* b0,
-                                      uint32_t* b1)
-{
-    int g = lane >> 2, t = lane & 3;
-    const __nv_bfloat16* row = w + (n0 + g) * ld + k0 + 2 * t;
-    *b0 = *reinterpret_cast<const uint32_t*>(row);
-    *b1 = *reinterpret_cast<const uint32_t*>(row + 8);
-}
-
-// B fragment (b0, b1) of tile (nt, kt) from a fragment-ordered image.
+// B fragment of an m16n8k16 MMA (k = 2t, 2t+1 | 2t+8, 2t+9; n = g), tile (nt, kt) of a
+// fragment-ordered image.
 __device__ __forceinline__ void LoadBFrag(const __nv_bfloat16* w, int n_tiles, int nt, int kt, int lane, uint32_t* b0,
                                           uint32_t* b1)
 {

@@ -18,7 +18,7 @@ namespace bbg
 namespace
 {
 
-constexpr int kTrainWarps = 6;
+constexpr int kTrainWarps = 12;
 
 // ------------------------------------------------------- tensor-core helpers
 
@@ -489,64 +489,79 @@ __device__ __forceinline__ void StageWeights(const __nv_bfloat16* wg, const floa
     __syncthreads();
 }
 
-// Gradient of -w log q(dir) w.r.t. the 40 raw outputs of one sample, and the
-// loss term (q: the vMF mixture of MakeMixture).
-__device__ __forceinline__ float MixtureNllGrad(const float* o, V3 dir, float weight, float* g)
+// The loss gradient of one sample, half of it: the calling lane takes lobes
+// 4 half .. 4 half + 3 of the row of 40 outputs and its neighbour (lane ^ 1) the
+// other four. Replaces the lane's 20 outputs by the gradient of -w log q(dir)
+// (q: the vMF mixture of MakeMixture) and returns the sample's loss term.
+__device__ __forceinline__ float MixtureNllGradHalf(float* o, V3 dir, float weight)
 {
-    VmfMixture m = MakeMixture(o);
-    float lp[kLobes];
+    constexpr int kHalf = kLobes / 2;
+    float lp[kHalf], logw[kHalf], kappa[kHalf], len[kHalf], cosm[kHalf];
+    V3 mu[kHalf];
     float mx = -INFINITY;
-    for (int j = 0; j < kLobes; ++j)
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j)
     {
-        float k = m.kappa[j];
-        lp[j] = m.logw[j] + VmfLogNorm(k) + k * (Dot(m.mu[j], dir) - 1.0f);
-        mx = fmaxf(mx, lp[j]);
+        mx = fmaxf(mx, o[5 * j]);
     }
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     float s = 0;
-    for (int j = 0; j < kLobes; ++j)
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j)
     {
-        s += expf(lp[j] - mx);
+        s += expf(o[5 * j] - mx);
     }
-    float logq = mx + logf(s);
-    for (int j = 0; j < kLobes; ++j)
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    const float lse = mx + logf(s);
+    float top = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j)
     {
-        float gamma = expf(lp[j] - logq); // responsibility
-        float pi = expf(m.logw[j]);
-        float k = m.kappa[j];
+        logw[j] = o[5 * j] - lse;
         V3 v{ o[5 * j + 1], o[5 * j + 2], o[5 * j + 3] };
-        float len = fmaxf(Length(v), 1e-6f);
-        float cosm = Dot(m.mu[j], dir);
-        V3 dm = (dir - m.mu[j] * cosm) * (gamma * k / len);
-        g[5 * j] = -weight * (gamma - pi);
-        g[5 * j + 1] = -weight * dm.x;
-        g[5 * j + 2] = -weight * dm.y;
-        g[5 * j + 3] = -weight * dm.z;
-        float r = o[5 * j + 4];
-        float two_k = 2.0f * k;
-        float dlogf_dlogk = 1.0f - two_k / expm1f(two_k) + k * (cosm - 1.0f);
-        bool clamped = r < kKappaLogMin || r > kKappaLogMax;
-        g[5 * j + 4] = clamped ? 0.0f : -weight * gamma * dlogf_dlogk;
+        len[j] = fmaxf(Length(v), 1e-6f);
+        mu[j] = v / len[j];
+        kappa[j] = expf(Clamp(o[5 * j + 4], kKappaLogMin, kKappaLogMax));
+        cosm[j] = Dot(mu[j], dir);
+        lp[j] = logw[j] + VmfLogNorm(kappa[j]) + kappa[j] * (cosm[j] - 1.0f);
+        top = fmaxf(top, lp[j]);
+    }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    float q = 0;
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j)
+    {
+        q += expf(lp[j] - top);
+    }
+    q += __shfl_xor_sync(0xffffffffu, q, 1);
+    const float logq = top + logf(q);
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j)
+    {
+        const float gamma = expf(lp[j] - logq); // responsibility
+        const float pi = expf(logw[j]);
+        const float k = kappa[j], r = o[5 * j + 4];
+        const V3 dm = (dir - mu[j] * cosm[j]) * (gamma * k / len[j]);
+        o[5 * j] = -weight * (gamma - pi);
+        o[5 * j + 1] = -weight * dm.x;
+        o[5 * j + 2] = -weight * dm.y;
+        o[5 * j + 3] = -weight * dm.z;
+        const float two_k = 2.0f * k;
+        const float dlogf_dlogk = 1.0f - two_k / expm1f(two_k) + k * (cosm[j] - 1.0f);
+        const bool clamped = r < kKappaLogMin || r > kKappaLogMax;
+        o[5 * j + 4] = clamped ? 0.0f : -weight * gamma * dlogf_dlogk;
     }
     return -weight * logq;
 }
 
-struct TrainWarp
-{
-    __nv_bfloat16 x[16 * kXLd];          // [sample][feature], padded rows
-    __nv_bfloat16 xt[kGuideIn * 16];     // [feature][sample]
-    __nv_bfloat16 h[3][16 * kGuideHidden];   // post-ReLU activations [sample][unit]
-    __nv_bfloat16 ht[3][kGuideHidden * 16];  // [unit][sample]
-    float y[16 * kGuideOut];             // outputs
-    __nv_bfloat16 dy[16 * kGuideOutPad]; // [sample][out], zero padded
-    __nv_bfloat16 dyt[kGuideOutPad * 16];
-    __nv_bfloat16 dh[16 * kGuideHidden];
-    __nv_bfloat16 dht[kGuideHidden * 16];
-};
-
 // Shared memory: weights (all images), packed biases, packed bias-gradient
-// accumulators, then one TrainWarp per warp.
-constexpr size_t kTrainSmem = size_t(kBfAll) * 2 + 2 * size_t(kCBias) * 4 + sizeof(TrainWarp) * kTrainWarps;
-static_assert((size_t(kBfAll) * 2 + 2 * size_t(kCBias) * 4) % 16 == 0, "TrainWarp alignment");
+// accumulators, then one tile buffer per warp: the 16 samples' features (BF16
+// [16][kXLd]), later their outputs and output gradients (float [16][kYLd]).
+constexpr int kYLd = 42; // even, for float2 accesses; rows start in distinct banks
+constexpr size_t kTrainTile = size_t(16) * kXLd * 2;
+static_assert(kTrainTile >= size_t(16) * kYLd * 4, "a tile buffer holds the outputs too");
+constexpr size_t kTrainSmem = size_t(kBfAll) * 2 + 2 * size_t(kCBias) * 4 + kTrainTile * kTrainWarps;
+static_assert((size_t(kBfAll) * 2 + 2 * size_t(kCBias) * 4) % 16 == 0, "tile buffer alignment");
 
 // Training scratch (global, bf16, one column per sample, row stride = the
 // batch capacity): the transposed layer inputs and output gradients that the
@@ -555,55 +570,36 @@ static_assert((size_t(kBfAll) * 2 + 2 * size_t(kCBias) * 4) % 16 == 0, "TrainWar
 constexpr int kRowX = 0, kRowH0 = 80, kRowH1 = 144, kRowH2 = 208, kRowDY = 272, kRowDZ2 = 320, kRowDZ1 = 384,
               kRowDZ0 = 448, kScratchRows = 512;
 
-// Copies a warp's [rows][16] bf16 block (16 samples) into scratch rows
-// row0.. at sample column col0 (16-byte stores).
-__device__ __forceinline__ void StoreColumns(const __nv_bfloat16* src, int rows, __nv_bfloat16* scratch, int64_t ld,
-                                             int row0, int64_t col0, int lane)
+// Writes a warp's A fragments (16 samples x 16 KT columns, BF16) transposed into
+// scratch rows row0.. at sample column col0: each 8 x 8 matrix of a fragment
+// is transposed in registers, so a lane stores two samples of one row.
+template <int KT>
+__device__ __forceinline__ void StoreTransposed(const uint32_t (&a)[KT][4], __nv_bfloat16* scratch, int64_t ld, int row0,
+                                                int64_t col0, int lane)
 {
-    for (int i = lane; i < 2 * rows; i += 32)
-    {
-        int r = i >> 1, half = i & 1;
-        uint4 v = *reinterpret_cast<const uint4*>(src + r * 16 + half * 8);
-        *reinterpret_cast<uint4*>(scratch + (int64_t(row0) + r) * ld + col0 + half * 8) = v;
-    }
-}
-
-// C fragments (16 rows x 64 cols) -> bf16 [16][64] and [64][16].
-__device__ __forceinline__ void StoreActs(const float (&acc)[8][4], __nv_bfloat16* rm, __nv_bfloat16* cm, int lane)
-{
-    int g = lane >> 2, t = lane & 3;
+    __nv_bfloat16* at = scratch + (int64_t(row0) + (lane >> 2)) * ld + col0 + 2 * (lane & 3);
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
+    for (int kt = 0; kt < KT; ++kt)
     {
 #pragma unroll
-        for (int half = 0; half < 2; ++half)
+        for (int i = 0; i < 4; ++i)
         {
-            int row = g + 8 * half;
-            int col = nt * 8 + 2 * t;
-            __nv_bfloat16 v0 = __float2bfloat16_rn(acc[nt][2 * half]);
-            __nv_bfloat16 v1 = __float2bfloat16_rn(acc[nt][2 * half + 1]);
-            rm[row * kGuideHidden + col] = v0;
-            rm[row * kGuideHidden + col + 1] = v1;
-            cm[col * 16 + row] = v0;
-            cm[(col + 1) * 16 + row] = v1;
+            uint32_t m;
+            asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(m) : "r"(a[kt][i]));
+            *reinterpret_cast<uint32_t*>(at + int64_t(kt * 16 + (i >> 1) * 8) * ld + (i & 1) * 8) = m;
         }
     }
 }
 
-// dZ = (dOut . W) masked by the ReLU of the layer's output h: A = dOut
-// [16][K] (ld lda), B = W^T stored [64][K]; writes dZ to dh / dht and adds the
-// column sums to the bias gradient.
+// dZ = (dOut . W) masked by the ReLU of the layer's output h (its A
+// fragments): A = dOut, B = W^T in fragment order; dZ as A fragments, its
+// column sums added to the lane's bias-gradient accumulators (columns
+// 8 nt + 2 t + {0, 1}, the lane's two rows).
 template <int KT>
-__device__ __forceinline__ void BackLayer(const __nv_bfloat16* dout, int lda, const __nv_bfloat16* wt, int ldw,
-                                          const __nv_bfloat16* h, __nv_bfloat16* dh, __nv_bfloat16* dht,
-                                          float* bias_grad, int lane)
+__device__ __forceinline__ void BackLayer(const uint32_t (&dout)[KT][4], const __nv_bfloat16* wt,
+                                          const uint32_t (&h)[4][4], uint32_t (&dz)[4][4], float (&bias)[8][2],
+                                          int lane)
 {
-    uint32_t a[KT][4];
-#pragma unroll
-    for (int kt = 0; kt < KT; ++kt)
-    {
-        LoadA(dout, lda, 0, kt * 16, lane, a[kt]);
-    }
     float acc[8][4];
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)
@@ -613,46 +609,56 @@ __device__ __forceinline__ void BackLayer(const __nv_bfloat16* dout, int lda, co
         for (int kt = 0; kt < KT; ++kt)
         {
             uint32_t b0, b1;
-            LoadB(wt, ldw, nt * 8, kt * 16, lane, &b0, &b1);
-            Mma16816(acc[nt], a[kt], b0, b1);
+            LoadBFrag(wt, 8, nt, kt, lane, &b0, &b1);
+            Mma16816(acc[nt], dout[kt], b0, b1);
         }
+        // h >= 0: an output passed the ReLU where its BF16 value is not zero.
+        const uint32_t h0 = h[nt >> 1][2 * (nt & 1)], h1 = h[nt >> 1][2 * (nt & 1) + 1];
+        acc[nt][0] = (h0 & 0x7fffu) ? acc[nt][0] : 0.0f;
+        acc[nt][1] = (h0 & 0x7fff0000u) ? acc[nt][1] : 0.0f;
+        acc[nt][2] = (h1 & 0x7fffu) ? acc[nt][2] : 0.0f;
+        acc[nt][3] = (h1 & 0x7fff0000u) ? acc[nt][3] : 0.0f;
+        bias[nt][0] += acc[nt][0] + acc[nt][2];
+        bias[nt][1] += acc[nt][1] + acc[nt][3];
     }
-    __syncwarp(); // every lane has read dout before dh is overwritten
-    int g = lane >> 2, t = lane & 3;
+    AccToA(acc, dz);
+}
+
+// Adds a layer's bias-gradient accumulators, summed over the warp's rows, to
+// the block's.
+__device__ __forceinline__ void FlushBias(const float (&bias)[8][2], float* out, int lane)
+{
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)
     {
-        float colsum0 = 0, colsum1 = 0;
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-        {
-            int row = g + 8 * half;
-            int col = nt * 8 + 2 * t;
-            float v0 = __bfloat162float(h[row * kGuideHidden + col]) > 0.0f ? acc[nt][2 * half] : 0.0f;
-            float v1 = __bfloat162float(h[row * kGuideHidden + col + 1]) > 0.0f ? acc[nt][2 * half + 1] : 0.0f;
-            colsum0 += v0;
-            colsum1 += v1;
-            __nv_bfloat16 b0 = __float2bfloat16_rn(v0), b1 = __float2bfloat16_rn(v1);
-            dh[row * kGuideHidden + col] = b0;
-            dh[row * kGuideHidden + col + 1] = b1;
-            dht[col * 16 + row] = b0;
-            dht[(col + 1) * 16 + row] = b1;
-        }
-        // Sum over the 8 row groups (lanes with equal t).
+        float s0 = bias[nt][0], s1 = bias[nt][1];
         for (int off = 4; off < 32; off <<= 1)
         {
-            colsum0 += __shfl_xor_sync(0xffffffffu, colsum0, off);
-            colsum1 += __shfl_xor_sync(0xffffffffu, colsum1, off);
+            s0 += __shfl_xor_sync(0xffffffffu, s0, off);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, off);
         }
-        if (g == 0)
+        if (lane < 4)
         {
-            atomicAdd(bias_grad + nt * 8 + 2 * t, colsum0);
-            atomicAdd(bias_grad + nt * 8 + 2 * t + 1, colsum1);
+            atomicAdd(out + nt * 8 + 2 * lane, s0);
+            atomicAdd(out + nt * 8 + 2 * lane + 1, s1);
         }
     }
-    __syncwarp();
 }
 
+// One training pass over a batch: a warp takes 16 samples at a time through
+// the network and back, with mma.sync on 16-row tiles: activations, ReLU masks
+// and gradients stay in registers as A fragments (AccToA turns a layer's
+// accumulators into the next one's operand), and only the features and the 40
+// outputs pass through a 2.8 KB buffer per warp. The weight gradients are
+// GEMMs over the whole batch and run on tcgen05 (GuideWeightGradTcKernel) from
+// the transposed operands that this kernel writes to the scratch.
+// Bound by the latency of a warp's chain (eight layers, the mixture's
+// exponentials), so warps in flight count: 12 per SM where the fragments'
+// copies in shared memory, in both orders, had allowed 6. With those copies,
+// a float atomic per sample and output for the bias gradients, 8-way bank
+// conflicts on the transposed weights and the mixture on half of the lanes, a
+// batch of 65,536 took 373 us on one B200; it takes 60 us (67 MB of scratch
+// written at 1.1 TB/s).
 __global__ void __launch_bounds__(32 * kTrainWarps) GuideTrainKernel(const float* raw, const float* dirs,
                                                                       const float* weights, const int32_t* n_dev,
                                                                       int64_t n_host, GuideBounds bounds,
@@ -664,7 +670,6 @@ __global__ void __launch_bounds__(32 * kTrainWarps) GuideTrainKernel(const float
     __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(smem);
     float* bs = reinterpret_cast<float*>(smem + size_t(kBfAll) * 2);
     float* bgs = bs + kCBias; // bias gradients, packed like bs
-    TrainWarp* tw = reinterpret_cast<TrainWarp*>(bgs + kCBias);
     StageWeights(wg, pg, ws, bs, kBfAll);
     for (int i = threadIdx.x; i < kCBias; i += blockDim.x)
     {
@@ -674,25 +679,23 @@ __global__ void __launch_bounds__(32 * kTrainWarps) GuideTrainKernel(const float
 
     const int64_t n = n_dev ? int64_t(*n_dev) : n_host;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    TrainWarp& W = tw[warp];
+    unsigned char* tile_buf = reinterpret_cast<unsigned char*>(bgs + kCBias) + size_t(warp) * kTrainTile;
+    __nv_bfloat16* x = reinterpret_cast<__nv_bfloat16*>(tile_buf); // [16][kXLd]
+    float* y = reinterpret_cast<float*>(tile_buf);                 // [16][kYLd]
     const int g = lane >> 2, t = lane & 3;
+    const int row = lane >> 1, half = lane & 1; // two lanes per sample
     float loss = 0;
+    float bias0[8][2] = {}, bias1[8][2] = {}, bias2[8][2] = {}; // bias gradients of the hidden layers
+    float bias3[2] = {};                                        // of outputs lane and 32 + lane
     const int64_t tiles = (n + 15) / 16;
     for (int64_t tile = int64_t(blockIdx.x) * kTrainWarps + warp; tile < tiles;
          tile += int64_t(gridDim.x) * kTrainWarps)
     {
-        // Features, both layouts.
+        const int64_t item = tile * 16 + row, col0 = tile * 16;
+        const bool valid = item < n;
         {
-            int row = lane >> 1, half = lane & 1;
-            int64_t item = tile * 16 + row;
-            bool valid = item < n;
             auto put = [&](int j, float v0, float v1) {
-                const int f = half * 40 + j;
-                const __nv_bfloat16 a = __float2bfloat16_rn(v0), b = __float2bfloat16_rn(v1);
-                W.x[row * kXLd + f] = a;
-                W.x[row * kXLd + f + 1] = b;
-                W.xt[f * 16 + row] = a;
-                W.xt[(f + 1) * 16 + row] = b;
+                *reinterpret_cast<uint32_t*>(x + row * kXLd + half * 40 + j) = PackBf16(v0, v1);
             };
             if (valid)
             {
@@ -712,93 +715,94 @@ __global__ void __launch_bounds__(32 * kTrainWarps) GuideTrainKernel(const float
                 }
             }
         }
+        V3 dir{ 0, 0, 1 };
+        float weight = 0;
+        if (valid)
+        {
+            dir = V3{ dirs[3 * item], dirs[3 * item + 1], dirs[3 * item + 2] };
+            weight = weights[item];
+        }
         __syncwarp();
 
-        // Forward, keeping activations.
-        uint32_t a0[5][4];
+        // Forward, the activations kept as A fragments.
+        uint32_t a0[5][4], h0[4][4], h1[4][4], h2[4][4];
 #pragma unroll
         for (int kt = 0; kt < 5; ++kt)
         {
-            LoadA(W.x, kXLd, 0, kt * 16, lane, a0[kt]);
+            LoadA(x, kXLd, 0, kt * 16, lane, a0[kt]);
         }
+        StoreTransposed(a0, scratch, ld, kRowX, col0, lane);
         float acc[8][4];
-        uint32_t a[4][4];
         HiddenLayer<5>(a0, ws + kBf0, bs + kCB0, lane, acc);
-        StoreActs(acc, W.h[0], W.ht[0], lane);
-        AccToA(acc, a);
-        HiddenLayer<4>(a, ws + kBf1, bs + kCB1, lane, acc);
-        StoreActs(acc, W.h[1], W.ht[1], lane);
-        AccToA(acc, a);
-        HiddenLayer<4>(a, ws + kBf2, bs + kCB2, lane, acc);
-        StoreActs(acc, W.h[2], W.ht[2], lane);
-        AccToA(acc, a);
+        AccToA(acc, h0);
+        StoreTransposed(h0, scratch, ld, kRowH0, col0, lane);
+        HiddenLayer<4>(h0, ws + kBf1, bs + kCB1, lane, acc);
+        AccToA(acc, h1);
+        StoreTransposed(h1, scratch, ld, kRowH1, col0, lane);
+        HiddenLayer<4>(h1, ws + kBf2, bs + kCB2, lane, acc);
+        AccToA(acc, h2);
+        StoreTransposed(h2, scratch, ld, kRowH2, col0, lane);
         float out[5][4];
-        OutputLayer(a, ws + kBf3, bs + kCB3, lane, out);
+        OutputLayer(h2, ws + kBf3, bs + kCB3, lane, out);
+        __syncwarp(); // every lane has read x, which y overlays
 #pragma unroll
         for (int nt = 0; nt < 5; ++nt)
         {
-#pragma unroll
-            for (int half = 0; half < 2; ++half)
-            {
-                int row = g + 8 * half;
-                W.y[row * kGuideOut + nt * 8 + 2 * t] = out[nt][2 * half];
-                W.y[row * kGuideOut + nt * 8 + 2 * t + 1] = out[nt][2 * half + 1];
-            }
+            *reinterpret_cast<float2*>(y + g * kYLd + nt * 8 + 2 * t) = make_float2(out[nt][0], out[nt][1]);
+            *reinterpret_cast<float2*>(y + (g + 8) * kYLd + nt * 8 + 2 * t) = make_float2(out[nt][2], out[nt][3]);
         }
         __syncwarp();
 
-        // Output gradient, one lane per sample.
-        if (lane < 16)
+        // Output gradients in place, two lanes per sample; zero past the batch.
         {
-            int64_t item = tile * 16 + lane;
-            float gy[kGuideOut];
-            if (item < n)
+            float* o = y + row * kYLd + (kGuideOut / 2) * half;
+            float gy[kGuideOut / 2];
+#pragma unroll
+            for (int k = 0; k < kGuideOut / 2; ++k)
             {
-                V3 dir{ dirs[3 * item], dirs[3 * item + 1], dirs[3 * item + 2] };
-                loss += MixtureNllGrad(W.y + lane * kGuideOut, dir, weights[item], gy);
+                gy[k] = o[k];
             }
-            else
+            const float term = MixtureNllGradHalf(gy, dir, weight);
+            loss += valid && half == 0 ? term : 0.0f;
+#pragma unroll
+            for (int k = 0; k < kGuideOut / 2; ++k)
             {
-                for (int k = 0; k < kGuideOut; ++k)
-                {
-                    gy[k] = 0;
-                }
-            }
-            for (int k = 0; k < kGuideOutPad; ++k)
-            {
-                float v = k < kGuideOut ? gy[k] : 0.0f;
-                __nv_bfloat16 b = __float2bfloat16_rn(v);
-                W.dy[lane * kGuideOutPad + k] = b;
-                W.dyt[k * 16 + lane] = b;
-                if (k < kGuideOut && v != 0.0f)
-                {
-                    atomicAdd(bgs + kCB3 + k, v);
-                }
+                o[k] = valid ? gy[k] : 0.0f;
             }
         }
         __syncwarp();
+        for (int k = 0; k < 16; ++k)
+        {
+            bias3[0] += y[k * kYLd + lane];
+            bias3[1] += lane < kGuideOut - 32 ? y[k * kYLd + 32 + lane] : 0.0f;
+        }
+        uint32_t dy[3][4];
+#pragma unroll
+        for (int kt = 0; kt < 3; ++kt)
+        {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const int c = kt * 16 + (i >> 1) * 8 + 2 * t;
+                float2 v = make_float2(0.0f, 0.0f);
+                if (kt * 16 + (i >> 1) * 8 < kGuideOut)
+                {
+                    v = *reinterpret_cast<const float2*>(y + (g + (i & 1) * 8) * kYLd + c);
+                }
+                dy[kt][i] = PackBf16(v.x, v.y);
+            }
+        }
+        StoreTransposed(dy, scratch, ld, kRowDY, col0, lane);
 
-        // Layer 3: dW3 += dY^T H3, dZ2 = (dY W3) * relu'(H3).
-        // The layer inputs and output gradients, transposed, go to the
-        // scratch columns of these 16 samples; the weight gradients are the
-        // GEMMs dW = dZ^T A over the whole batch (GuideWeightGradTcKernel).
-        const int64_t col0 = tile * 16;
-        StoreColumns(W.xt, kGuideIn, scratch, ld, kRowX, col0, lane);
-        StoreColumns(W.ht[0], kGuideHidden, scratch, ld, kRowH0, col0, lane);
-        StoreColumns(W.ht[1], kGuideHidden, scratch, ld, kRowH1, col0, lane);
-        StoreColumns(W.ht[2], kGuideHidden, scratch, ld, kRowH2, col0, lane);
-        StoreColumns(W.dyt, kGuideOutPad, scratch, ld, kRowDY, col0, lane);
         // dZ2 = (dY W3) * relu'(H2), then dZ1, dZ0 likewise.
-        BackLayer<3>(W.dy, kGuideOutPad, ws + kBfT3, kGuideOutPad, W.h[2], W.dh, W.dht, bgs + kCB2, lane);
-        __syncwarp();
-        StoreColumns(W.dht, kGuideHidden, scratch, ld, kRowDZ2, col0, lane);
-        BackLayer<4>(W.dh, kGuideHidden, ws + kBfT2, kGuideHidden, W.h[1], W.dh, W.dht, bgs + kCB1, lane);
-        __syncwarp();
-        StoreColumns(W.dht, kGuideHidden, scratch, ld, kRowDZ1, col0, lane);
-        BackLayer<4>(W.dh, kGuideHidden, ws + kBfT1, kGuideHidden, W.h[0], W.dh, W.dht, bgs + kCB0, lane);
-        __syncwarp();
-        StoreColumns(W.dht, kGuideHidden, scratch, ld, kRowDZ0, col0, lane);
-        __syncwarp();
+        uint32_t dz[4][4], dz1[4][4];
+        BackLayer<3>(dy, ws + kBfT3, h2, dz, bias2, lane);
+        StoreTransposed(dz, scratch, ld, kRowDZ2, col0, lane);
+        BackLayer<4>(dz, ws + kBfT2, h1, dz1, bias1, lane);
+        StoreTransposed(dz1, scratch, ld, kRowDZ1, col0, lane);
+        BackLayer<4>(dz1, ws + kBfT1, h0, dz, bias0, lane);
+        StoreTransposed(dz, scratch, ld, kRowDZ0, col0, lane);
+        __syncwarp(); // every lane has read y, which the next tile's x overlays
     }
     for (int off = 16; off > 0; off >>= 1)
     {
@@ -807,6 +811,14 @@ __global__ void __launch_bounds__(32 * kTrainWarps) GuideTrainKernel(const float
     if (lane == 0 && loss != 0.0f)
     {
         atomicAdd(loss_out, loss);
+    }
+    FlushBias(bias0, bgs + kCB0, lane);
+    FlushBias(bias1, bgs + kCB1, lane);
+    FlushBias(bias2, bgs + kCB2, lane);
+    atomicAdd(bgs + kCB3 + lane, bias3[0]);
+    if (lane < kGuideOut - 32)
+    {
+        atomicAdd(bgs + kCB3 + 32 + lane, bias3[1]);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kCBias; i += blockDim.x)
@@ -1084,20 +1096,17 @@ __global__ void GuideConvertKernel(const float* params, __nv_bfloat16* w)
             int k = (tile / n_tiles) * 16 + 2 * (lane & 3) + (e & 1) + 8 * (e >> 1);
             v = params[src + n * n_in + k];
         }
-        else if (i < kBfT2)
-        {
-            int j = i - kBfT1, r = j / kGuideHidden, c = j % kGuideHidden; // W1^T[r][c] = W1[c][r]
-            v = params[kW1 + c * kGuideHidden + r];
-        }
-        else if (i < kBfT3)
-        {
-            int j = i - kBfT2, r = j / kGuideHidden, c = j % kGuideHidden;
-            v = params[kW2 + c * kGuideHidden + r];
-        }
         else
         {
-            int j = i - kBfT3, r = j / kGuideOutPad, c = j % kGuideOutPad; // W3^T[r][c] = W3[c][r]
-            v = c < kGuideOut ? params[kW3 + c * kGuideHidden + r] : 0.0f;
+            // Transposed weights in fragment order (see kBfT1): n is the input
+            // unit, k the output unit.
+            const int base = i < kBfT2 ? kBfT1 : i < kBfT3 ? kBfT2 : kBfT3;
+            const int src = i < kBfT2 ? kW1 : i < kBfT3 ? kW2 : kW3;
+            const int n_out = i < kBfT3 ? kGuideHidden : kGuideOut;
+            const int j = i - base, e = j & 3, lane = (j >> 2) & 31, tile = j >> 7;
+            const int n = (tile % (kGuideHidden / 8)) * 8 + (lane >> 2);
+            const int k = (tile / (kGuideHidden / 8)) * 16 + 2 * (lane & 3) + (e & 1) + 8 * (e >> 1);
+            v = k < n_out ? params[src + k * kGuideHidden + n] : 0.0f;
         }
         w[i] = __float2bfloat16_rn(v);
     }
