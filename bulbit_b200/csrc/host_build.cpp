@@ -173,7 +173,17 @@ bbg_status CheckGeometry(const bbg_geometry* g)
     {
         return Fail(BBG_ERR_INVALID_ARG, "geometry: triangles without indices or positions");
     }
-    for (int32_t t = 0; t < 3 * g->n_triangles; ++t)
+    // The largest index as unsigned first (a negative one is larger than any
+    // count); the loop that names the offender only where there is one.
+    uint32_t worst[4] = { 0, 0, 0, 0 };
+    const int64_t n_indices = 3 * int64_t(g->n_triangles);
+    for (int64_t t = 0; t < n_indices; ++t)
+    {
+        worst[t & 3] = std::max(worst[t & 3], uint32_t(g->tri_indices[t]));
+    }
+    const bool in_range =
+        n_indices == 0 || std::max({ worst[0], worst[1], worst[2], worst[3] }) < uint32_t(g->n_vertices);
+    for (int64_t t = 0; !in_range && t < n_indices; ++t)
     {
         if (g->tri_indices[t] < 0 || g->tri_indices[t] >= g->n_vertices)
         {

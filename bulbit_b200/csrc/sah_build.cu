@@ -1246,8 +1246,10 @@ __global__ void SahWide8WriteKernel(const bbg_bvh_node* nd, const uint8_t* split
 // The 8-wide collapse of the depth-first node array on the device, level by
 // level (the host reads each level's size back). Leaves the layout unbuilt if
 // a leaf cannot be encoded or the tree exceeds the layout's limits, as the
-// host collapse does.
-bbg_status SahWide8(bbg_accel* a, const bbg_bvh_node* nd, int32_t n_nodes, int sms)
+// host collapse does. scratch: scratch_bytes of device memory for its
+// temporaries, which are allocated instead where they do not fit.
+bbg_status SahWide8(bbg_accel* a, const bbg_bvh_node* nd, int32_t n_nodes, int sms, uint8_t* scratch,
+                    size_t scratch_bytes)
 {
     // Every wide node stands for a distinct interior binary node (or the
     // root leaf), so that many always suffice; the layout encodes at most
@@ -1256,30 +1258,55 @@ bbg_status SahWide8(bbg_accel* a, const bbg_bvh_node* nd, int32_t n_nodes, int s
     const int32_t capacity = std::max(interior, 1);
     constexpr int64_t kMaxWide = (int64_t(1) << 23) - 1;
     cudaStream_t st = a->stream;
-    DevBuf<int32_t> w2b, inner, offsets, flag, parent, arrivals;
-    DevBuf<float> cost;
-    DevBuf<uint8_t> split;
-    BBG_TRY(parent.alloc(size_t(n_nodes)));
-    BBG_TRY(arrivals.alloc(size_t(n_nodes)));
-    BBG_TRY(cost.alloc(8 * size_t(n_nodes)));
-    BBG_TRY(split.alloc(8 * size_t(n_nodes)));
-    BBG_CUDA(cudaMemsetAsync(arrivals.p, 0, sizeof(int32_t) * size_t(n_nodes), st));
-    BBG_CUDA(cudaMemsetAsync(cost.p, 0, sizeof(float) * 8 * size_t(n_nodes), st)); // leaves cost 0
-    BBG_CUDA(cudaMemsetAsync(split.p, 0, 8 * size_t(n_nodes), st));
-    SahPlanParentKernel<<<GridFor(n_nodes, 256, sms), 256, 0, st>>>(nd, n_nodes, parent.p);
-    SahPlanKernel<<<GridFor(n_nodes, 256, sms), 256, 0, st>>>(nd, n_nodes, parent.p, arrivals.p, cost.p, split.p);
-    BBG_CUDA(cudaGetLastError());
-    BBG_TRY(w2b.alloc(size_t(capacity)));
-    BBG_TRY(inner.alloc(size_t(capacity) + 1));
-    BBG_TRY(offsets.alloc(size_t(capacity) + 1));
-    BBG_TRY(flag.alloc(1));
-    BBG_TRY(a->wide8.alloc(6 * size_t(capacity)));
-    BBG_CUDA(cudaMemsetAsync(w2b.p, 0, sizeof(int32_t), st)); // wide node 0 = binary root 0
-    BBG_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int32_t), st));
     size_t scan_bytes = 0;
-    BBG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, inner.p, offsets.p, capacity + 1, st));
-    DevBuf<uint8_t> scan_tmp;
-    BBG_TRY(scan_tmp.alloc(std::max<size_t>(scan_bytes, 1)));
+    int32_t* none = nullptr;
+    BBG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, none, none, capacity + 1, st));
+    int32_t *w2b = nullptr, *inner = nullptr, *offsets = nullptr, *flag = nullptr, *parent = nullptr, *arrivals = nullptr;
+    float* cost = nullptr;
+    uint8_t *split = nullptr, *scan_tmp = nullptr;
+    const struct
+    {
+        void** ptr;
+        size_t bytes;
+    } pieces[] = {
+        { reinterpret_cast<void**>(&parent), size_t(n_nodes) * sizeof(int32_t) },
+        { reinterpret_cast<void**>(&arrivals), size_t(n_nodes) * sizeof(int32_t) },
+        { reinterpret_cast<void**>(&cost), 8 * size_t(n_nodes) * sizeof(float) },
+        { reinterpret_cast<void**>(&split), 8 * size_t(n_nodes) },
+        { reinterpret_cast<void**>(&w2b), size_t(capacity) * sizeof(int32_t) },
+        { reinterpret_cast<void**>(&inner), (size_t(capacity) + 1) * sizeof(int32_t) },
+        { reinterpret_cast<void**>(&offsets), (size_t(capacity) + 1) * sizeof(int32_t) },
+        { reinterpret_cast<void**>(&flag), sizeof(int32_t) },
+        { reinterpret_cast<void**>(&scan_tmp), std::max<size_t>(scan_bytes, 1) },
+    };
+    size_t need = 0;
+    for (const auto& pc : pieces)
+    {
+        need += (pc.bytes + 255) / 256 * 256;
+    }
+    DevBuf<uint8_t> own;
+    if (need > scratch_bytes)
+    {
+        BBG_TRY(own.alloc(need));
+        scratch = own.p;
+    }
+    {
+        size_t at = 0;
+        for (const auto& pc : pieces)
+        {
+            *pc.ptr = scratch + at;
+            at += (pc.bytes + 255) / 256 * 256;
+        }
+    }
+    BBG_CUDA(cudaMemsetAsync(arrivals, 0, sizeof(int32_t) * size_t(n_nodes), st));
+    BBG_CUDA(cudaMemsetAsync(cost, 0, sizeof(float) * 8 * size_t(n_nodes), st)); // leaves cost 0
+    BBG_CUDA(cudaMemsetAsync(split, 0, 8 * size_t(n_nodes), st));
+    SahPlanParentKernel<<<GridFor(n_nodes, 256, sms), 256, 0, st>>>(nd, n_nodes, parent);
+    SahPlanKernel<<<GridFor(n_nodes, 256, sms), 256, 0, st>>>(nd, n_nodes, parent, arrivals, cost, split);
+    BBG_CUDA(cudaGetLastError());
+    BBG_TRY(a->wide8.alloc(6 * size_t(capacity)));
+    BBG_CUDA(cudaMemsetAsync(w2b, 0, sizeof(int32_t), st)); // wide node 0 = binary root 0
+    BBG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int32_t), st));
     int32_t begin = 0, end = 1, depth = 0;
     while (begin < end)
     {
@@ -1289,20 +1316,20 @@ bbg_status SahWide8(bbg_accel* a, const bbg_bvh_node* nd, int32_t n_nodes, int s
             return BBG_OK;
         }
         const int32_t m = end - begin;
-        SahWide8CountKernel<<<GridFor(m, 128, sms), 128, 0, st>>>(nd, split.p, w2b.p, begin, end, inner.p, flag.p);
+        SahWide8CountKernel<<<GridFor(m, 128, sms), 128, 0, st>>>(nd, split, w2b, begin, end, inner, flag);
         // offsets[m], the level's total, needs inner[m] = 0.
-        BBG_CUDA(cudaMemsetAsync(inner.p + m, 0, sizeof(int32_t), st));
-        BBG_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp.p, scan_bytes, inner.p, offsets.p, m + 1, st));
+        BBG_CUDA(cudaMemsetAsync(inner + m, 0, sizeof(int32_t), st));
+        BBG_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, inner, offsets, m + 1, st));
         int32_t state[2] = { 0, 0 };
-        BBG_CUDA(cudaMemcpyAsync(&state[0], offsets.p + m, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        BBG_CUDA(cudaMemcpyAsync(&state[1], flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        BBG_CUDA(cudaMemcpyAsync(&state[0], offsets + m, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        BBG_CUDA(cudaMemcpyAsync(&state[1], flag, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         BBG_CUDA(cudaStreamSynchronize(st));
         if (state[1] != 0 || int64_t(end) + state[0] > std::min<int64_t>(capacity, kMaxWide))
         {
             a->wide8.reset();
             return BBG_OK;
         }
-        SahWide8WriteKernel<<<GridFor(m, 128, sms), 128, 0, st>>>(nd, split.p, w2b.p, begin, end, offsets.p,
+        SahWide8WriteKernel<<<GridFor(m, 128, sms), 128, 0, st>>>(nd, split, w2b, begin, end, offsets,
                                                                   a->wide8.p);
         BBG_CUDA(cudaGetLastError());
         begin = end;
@@ -1500,7 +1527,7 @@ bbg_status BuildSahOnDevice(bbg_accel* a, int32_t n, const float4* ref_box, cons
     a->n_slots = n;
     std::memcpy(a->bounds, root_node.bmin, 3 * sizeof(float));
     std::memcpy(a->bounds + 3, root_node.bmax, 3 * sizeof(float));
-    BBG_TRY(SahWide8(a, nd, n_nodes, sms));
+    BBG_TRY(SahWide8(a, nd, n_nodes, sms, arena.p, total)); // the build's own temporaries are spent
     BBG_CUDA(cudaStreamSynchronize(st));
     return BBG_OK;
 }
