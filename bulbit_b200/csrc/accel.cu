@@ -8,7 +8,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <thread>
+#include <tuple>
 
 namespace bbg
 {
@@ -45,11 +48,29 @@ int CurrentSmCount()
     return sms;
 }
 
+// Asked of the runtime once per kernel, launch shape and device: a render asks
+// for three dozen of them, a query for one, each some microseconds.
 int PersistentGrid(const void* kernel, int block, size_t smem)
 {
+    static std::mutex mutex;
+    static std::map<std::tuple<const void*, int, size_t, int>, int> grids;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const std::tuple<const void*, int, size_t, int> key{ kernel, block, smem, dev };
+    std::lock_guard<std::mutex> lock(mutex);
+    auto it = grids.find(key);
+    if (it != grids.end())
+    {
+        return it->second;
+    }
     int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
-    return CurrentSmCount() * std::max(per_sm, 1);
+    const bool known = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) == cudaSuccess;
+    const int grid = CurrentSmCount() * std::max(per_sm, 1);
+    if (known)
+    {
+        grids[key] = grid;
+    }
+    return grid;
 }
 
 // Reference-order traversal (and the counting run): one thread per ray,
@@ -136,6 +157,17 @@ __global__ void __launch_bounds__(kTraceBlock, TraceMinBlocks(kTraceBlock, WIDE)
     {
         TracePersistent<ANY>(a, n, next, src);
     }
+    // The last block to finish clears the work counter for the next launch
+    // (next[1] counts finished blocks), which saves a memset per query.
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        if (atomicAdd(next + 1, 1) == int32_t(gridDim.x) - 1)
+        {
+            next[0] = 0;
+            next[1] = 0;
+        }
+    }
 }
 
 template <bool ANY>
@@ -175,7 +207,6 @@ static bbg_status LaunchTrace(bbg_accel* a, const float4* rays, int64_t n, float
         for (int64_t c = 0; c < n; c += chunk)
         {
             int32_t m = int32_t(std::min(chunk, n - c));
-            BBG_CUDA(cudaMemsetAsync(a->work.p, 0, sizeof(int32_t), stream));
             k<<<grid, kTraceBlock, 0, stream>>>(a->view(), rays + 2 * c, m, hits ? hits + c : nullptr,
                                                 occ ? occ + c : nullptr, a->work.p);
         }
@@ -519,7 +550,8 @@ bbg_status CreateAccel(const bbg_geometry* g, const bbg_bvh* bvh, bbg_accel* a, 
         BBG_TRY(copies.Join());
         BBG_TRY(shading.Join());
         BBG_TRY(a->counters.alloc(2));
-        BBG_TRY(a->work.alloc(1));
+        BBG_TRY(a->work.alloc(2));
+        BBG_CUDA(cudaMemsetAsync(a->work.p, 0, 2 * sizeof(int32_t), a->stream));
         BBG_CUDA(cudaStreamSynchronize(a->stream));
         return BBG_OK;
     }
@@ -604,7 +636,8 @@ bbg_status CreateAccel(const bbg_geometry* g, const bbg_bvh* bvh, bbg_accel* a, 
     BBG_TRY(UploadGeometry(a, g));
     BBG_TRY(UploadShading(a, g, a->stream));
     BBG_TRY(a->counters.alloc(2));
-    BBG_TRY(a->work.alloc(1));
+    BBG_TRY(a->work.alloc(2));
+    BBG_CUDA(cudaMemsetAsync(a->work.p, 0, 2 * sizeof(int32_t), a->stream));
     BBG_CUDA(cudaStreamSynchronize(a->stream));
     return BBG_OK;
 }

@@ -333,14 +333,44 @@ __global__ void __launch_bounds__(kBlock) RaygenKernel(Scenes sc, WaveDev w)
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
         w.counts[0] = int32_t(n);
-        w.counts[1] = 0;
-        w.counts[2] = 0;
+        w.counts[3] = 0; // the first level's closest-hit pass
     }
 }
 
 // ---------------------------------------------------------------- intersect
 //
 // In a batch, each work item is traced in its own scene's tree (View).
+//
+// A level's counters are cleared by the passes around their use, not by a
+// launch of their own (2 us a level, a twentieth of a small frame): the
+// closest-hit pass clears what the level's later passes count with (the level
+// before is done with it), and shading, which follows it, its work counter.
+
+__device__ __forceinline__ void ClearLevelCounters(const WaveDev& w, int parity)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        w.counts[parity ^ 1] = 0; // next level's ray queue
+        w.counts[2] = 0;          // shadow queue
+        w.counts[4] = 0;          // work counter of the shadow pass
+        w.counts[5] = 0;          // guide queries
+        if (w.sorted)
+        {
+            for (int k = 0; k < 2 * kShadeKinds; ++k)
+            {
+                w.sort_counts[k] = 0;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void ClearClosestCounter(const WaveDev& w)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        w.counts[3] = 0;
+    }
+}
 
 // Work items of the closest-hit pass: queue entry j -> its path's ray.
 struct ClosestSrc
@@ -433,6 +463,7 @@ __global__ void __launch_bounds__(BLOCK, TraceMinBlocks(BLOCK, WIDE)) ClosestKer
     {
         atomicAdd(w.stats, (unsigned long long)n);
     }
+    ClearLevelCounters(w, parity);
     const SceneDev& s = sc.Scene(0);
     if constexpr (kIsBatch<Scenes>)
     {
@@ -657,6 +688,7 @@ __global__ void __launch_bounds__(kBlock, BBG_SHADE_MIN_BLOCKS) ShadeKernel(Scen
     const int32_t* q = w.sorted ? w.sorted : w.queue[parity];
     int32_t* q_next = w.queue[parity ^ 1];
     const int32_t n = w.counts[parity];
+    ClearClosestCounter(w);
 
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
     {
@@ -1022,6 +1054,7 @@ __global__ void __launch_bounds__(kBlock, BBG_SHADE_MIN_BLOCKS) GuidedShadeA(Sce
     const int32_t* q = w.sorted ? w.sorted : w.queue[parity];
     int32_t* q_next = w.queue[parity ^ 1];
     const int32_t n = w.counts[parity];
+    ClearClosestCounter(w);
     for (int32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
     {
         int32_t slot = q[j];
@@ -1419,25 +1452,13 @@ __global__ void GuideNormalizeKernel(GuideDev g)
     }
 }
 
-// Clears the next level's ray queue, the shadow queue, the work counters of
-// the persistent closest-hit and shadow passes and the guide-query queue.
-__global__ void ResetKernel(WaveDev w, int parity)
-{
-    w.counts[parity ^ 1] = 0;
-    w.counts[2] = 0;
-    w.counts[3] = 0;
-    w.counts[4] = 0;
-    w.counts[5] = 0;
-    if (w.sorted)
-    {
-        for (int k = 0; k < 2 * kShadeKinds; ++k)
-        {
-            w.sort_counts[k] = 0;
-        }
-    }
-}
-
 // ---------------------------------------------------------------- shading order
+
+__host__ __device__ __forceinline__ int32_t MaterialKind(const MaterialDev& md)
+{
+    const int32_t type = md.type < 0 ? 0 : (md.type > 3 ? 3 : md.type);
+    return 2 + 2 * type + (md.ms ? 1 : 0);
+}
 
 template <class Scenes>
 __device__ __forceinline__ int32_t ShadeKind(const Scenes& sc, const WaveDev& w, int32_t slot)
@@ -1453,8 +1474,7 @@ __device__ __forceinline__ int32_t ShadeKind(const Scenes& sc, const WaveDev& w,
     {
         return 1;
     }
-    const MaterialDev& md = s.materials[m];
-    return 2 + 2 * min(max(md.type, 0), 3) + (md.ms ? 1 : 0);
+    return MaterialKind(s.materials[m]);
 }
 
 // Counting sort of a level's queue by shading kind, pass 1: the kind of every
@@ -1821,6 +1841,10 @@ struct bbg_integrator
     bool graph_shade_sort = false;
     // Shading order of the current render (params.shade_order).
     bool shade_sort = true;
+    // The one kind (ShadeKind) of every primitive's material, -1 if there are
+    // several: with one there is nothing to sort a level by but its escaped
+    // rays, and the two sorting passes cost more than those.
+    int32_t only_kind = -1;
     DevBuf<int32_t> sorted, sort_counts;
     DevBuf<uint8_t> keys;
     // Launch shape of the traversal passes (index into kShapes) and wave size
@@ -2174,7 +2198,6 @@ bbg_status EnqueueLevel(const Grids& gr, const SceneDev& s, const WaveDev& w, co
                         int shape, cudaStream_t st)
 {
     const OneScene one{ s, FilmDev{} };
-    ResetKernel<<<1, 1, 0, st>>>(w, parity);
     LaunchTrace(shape, gr, one, w, parity, false, st);
     if (gc.guide)
     {
@@ -2270,7 +2293,7 @@ bbg_status PrepareSamplerAndFilter(bbg_integrator* I, const bbg_camera* cam, con
     {
         return Fail(BBG_ERR_INVALID_ARG, "shade_order %d", p->shade_order);
     }
-    I->shade_sort = p->shade_order == BBG_SHADE_SORTED;
+    I->shade_sort = p->shade_order == BBG_SHADE_SORTED && I->only_kind < 0;
     if (p->sampler != BBG_SAMPLER_INDEPENDENT &&
         (p->sampler != BBG_SAMPLER_STRATIFIED || p->x_samples <= 0 || p->spp % p->x_samples != 0))
     {
@@ -2615,6 +2638,7 @@ bbg_status CreateIntegrator(bbg_integrator* I, bbg_accel* a, const int32_t* prim
         }
     }
     std::vector<int4> info(size_t(a->n_prims));
+    bool several = false; // materials of several kinds
     for (int32_t i = 0; i < a->n_prims; ++i)
     {
         int32_t m = prim_material ? prim_material[i] : -1;
@@ -2623,7 +2647,11 @@ bbg_status CreateIntegrator(bbg_integrator* I, bbg_accel* a, const int32_t* prim
             return Fail(BBG_ERR_INVALID_ARG, "primitive %d names material %d of %d", i, m, n_mats);
         }
         info[i] = make_int4(a->host_prim_shape[i].x, a->host_prim_shape[i].y, m, -1);
+        const int32_t kind = m < 0 ? 1 : MaterialKind(md[m]);
+        I->only_kind = i == 0 || kind == I->only_kind ? kind : -1;
+        several = several || I->only_kind < 0;
     }
+    I->only_kind = several ? -1 : I->only_kind;
 
     // Geometry view for the host-side light set-up.
     bbg_geometry g{};
@@ -2708,7 +2736,6 @@ using BatchGrids = GridsT<SceneTable>;
 bbg_status EnqueueBatchLevel(const BatchGrids& gr, const SceneTable& t, const WaveDev& w, const GuideCtx& gc,
                              const GuideGroup* groups, int parity, int shape, cudaStream_t st)
 {
-    ResetKernel<<<1, 1, 0, st>>>(w, parity);
     LaunchTrace(shape, gr, t, w, parity, false, st);
     if (gc.guide)
     {
@@ -2866,7 +2893,12 @@ bbg_status RenderBatch(bbg_batch* B, int32_t n, bbg_integrator* const* integrato
     {
         return Fail(BBG_ERR_INVALID_ARG, "bbg_batch_render: shade_order %d", params[0].shade_order);
     }
-    E->shade_sort = params[0].shade_order == BBG_SHADE_SORTED;
+    bool one_kind = true;
+    for (int32_t i = 0; i < n; ++i)
+    {
+        one_kind = one_kind && integrators[i]->only_kind >= 0 && integrators[i]->only_kind == integrators[0]->only_kind;
+    }
+    E->shade_sort = params[0].shade_order == BBG_SHADE_SORTED && !one_kind;
     BBG_TRY(B->scenes.upload(B->host_scenes.data(), B->host_scenes.size(), st));
     BBG_TRY(B->films.upload(B->host_films.data(), B->host_films.size(), st));
     BBG_TRY(B->pixel_start.upload(B->host_pixel_start.data(), B->host_pixel_start.size(), st));
