@@ -40,7 +40,7 @@ struct RayQ
     V3 inv_box;       // finite 1 / d of the ordered and 8-wide box tests (BoxInverse)
     V3 dn;            // d after Vector3::Normalize (triangle test)
     float l;          // length returned by that Normalize
-    V3 oinv;          // o * inv_box, for the fused slab test of the ordered traversal
+    V3 o_near, o_far; // o * inv_box moved outward, for the fused slab test of the ordered traversal
     int neg[3];       // inv_dir < 0
 };
 
@@ -53,12 +53,29 @@ struct RayQ
 // 1,310,734-triangle Cornell scene one such ray opened 3,200 wide nodes and
 // tested 13,553 triangles (the mean ray: 13 and 21) and kept its launch alive
 // long after the other rays had finished (2^21 incoherent rays: 8.4 ms, now
-// 2.05 ms). The ray strays less than 1e-18 of its length from the
-// given one, far inside the boxes' padding, so no primitive that the reference
-// reaches is culled; a direction of length zero keeps its infinities.
+// 2.05 ms). The ray strays less than 1e-18 of its length from the given one;
+// where it runs in a box's face, which the reference's NaN never culls, the
+// tests move their planes outward by more than the face's distance comes out
+// at (SlabMargin, IntersectNode8), so no primitive that the reference reaches
+// is culled; a direction of length zero keeps its infinities.
 __device__ __forceinline__ float BoxInverse(float d, float least)
 {
     return 1 / (fabsf(d) < least ? copysignf(least, d) : d);
+}
+
+// How far the ordered traversal's slab test, plane * inv - o_inv with o_inv =
+// o * inv rounded, moves its planes outward. At a plane through the origin's
+// own coordinate all that is left is the rounding of o_inv (half an ulp, and
+// as much again where the margin is added), of either sign and, with a
+// reciprocal of 1e18, larger than any distance along the ray: without a
+// margin the box of a face at coordinate 100 was culled for half of the rays
+// that run in it (below 32 the boxes' padding of 10 epsilon hid it). The first
+// term is twice that rounding; the second, half an epsilon of length, keeps
+// the interval open at coordinate 0, where boxes without padding (spheres')
+// have faces and the first term vanishes.
+__device__ __forceinline__ float SlabMargin(float o_inv, float inv)
+{
+    return __fmaf_rn(fabsf(o_inv), 0x1p-22f, fabsf(inv) * 0x1p-24f);
 }
 
 __device__ __forceinline__ RayQ MakeRayQ(V3 o, V3 d)
@@ -74,7 +91,10 @@ __device__ __forceinline__ RayQ MakeRayQ(V3 o, V3 d)
     q.l = NormalizeInPlace(q.dn);
     const float least = 1e-18f * fmaxf(fabsf(d.x), fmaxf(fabsf(d.y), fabsf(d.z)));
     q.inv_box = V3{ BoxInverse(d.x, least), BoxInverse(d.y, least), BoxInverse(d.z, least) };
-    q.oinv = V3{ o.x * q.inv_box.x, o.y * q.inv_box.y, o.z * q.inv_box.z };
+    const V3 oi{ o.x * q.inv_box.x, o.y * q.inv_box.y, o.z * q.inv_box.z };
+    const V3 m{ SlabMargin(oi.x, q.inv_box.x), SlabMargin(oi.y, q.inv_box.y), SlabMargin(oi.z, q.inv_box.z) };
+    q.o_near = oi + m;
+    q.o_far = oi - m;
     return q;
 }
 
@@ -308,21 +328,20 @@ __device__ __forceinline__ TraceResult TraceReference(const AccelView& a, const 
 }
 
 // Slab test of one child box: [entry, exit] of the ray within the box and
-// within [t_min, t_max], with the reference's per-axis arithmetic
-// (bound - o) * (1/d) (include/bulbit/bounding_box.h:448-480).
+// within [t_min, t_max] (include/bulbit/bounding_box.h:448-480).
 __device__ __forceinline__ bool SlabTest(float lx, float ly, float lz, float hx, float hy, float hz, const RayQ& q,
                                          float t_min, float t_max, float* entry)
 {
-    // bound * (1/d) - o * (1/d) in one fused multiply-add per plane. It may
-    // round differently from the reference's (bound - o) * (1/d); it only
-    // decides which boxes are opened, and triangle boxes are padded by
-    // 10 epsilon (src/geometry/triangle.cpp:42), far beyond that rounding.
-    float x0 = __fmaf_rn(q.neg[0] ? hx : lx, q.inv_box.x, -q.oinv.x);
-    float x1 = __fmaf_rn(q.neg[0] ? lx : hx, q.inv_box.x, -q.oinv.x);
-    float y0 = __fmaf_rn(q.neg[1] ? hy : ly, q.inv_box.y, -q.oinv.y);
-    float y1 = __fmaf_rn(q.neg[1] ? ly : hy, q.inv_box.y, -q.oinv.y);
-    float z0 = __fmaf_rn(q.neg[2] ? hz : lz, q.inv_box.z, -q.oinv.z);
-    float z1 = __fmaf_rn(q.neg[2] ? lz : hz, q.inv_box.z, -q.oinv.z);
+    // bound * (1/d) - o * (1/d) in one fused multiply-add per plane. It rounds
+    // differently from the reference's (bound - o) * (1/d); it only decides
+    // which boxes are opened, and the planes are moved outward by more than
+    // o * (1/d) can be off (SlabMargin).
+    float x0 = __fmaf_rn(q.neg[0] ? hx : lx, q.inv_box.x, -q.o_near.x);
+    float x1 = __fmaf_rn(q.neg[0] ? lx : hx, q.inv_box.x, -q.o_far.x);
+    float y0 = __fmaf_rn(q.neg[1] ? hy : ly, q.inv_box.y, -q.o_near.y);
+    float y1 = __fmaf_rn(q.neg[1] ? ly : hy, q.inv_box.y, -q.o_far.y);
+    float z0 = __fmaf_rn(q.neg[2] ? hz : lz, q.inv_box.z, -q.o_near.z);
+    float z1 = __fmaf_rn(q.neg[2] ? lz : hz, q.inv_box.z, -q.o_far.z);
     float t0 = fmaxf(fmaxf(x0, y0), fmaxf(z0, t_min));
     float t1 = fminf(fminf(x1, y1), fminf(z1, t_max));
     *entry = t0;
