@@ -157,17 +157,6 @@ __global__ void __launch_bounds__(kTraceBlock, TraceMinBlocks(kTraceBlock, WIDE)
     {
         TracePersistent<ANY>(a, n, next, src);
     }
-    // The last block to finish clears the work counter for the next launch
-    // (next[1] counts finished blocks), which saves a memset per query.
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        if (atomicAdd(next + 1, 1) == int32_t(gridDim.x) - 1)
-        {
-            next[0] = 0;
-            next[1] = 0;
-        }
-    }
 }
 
 template <bool ANY>
@@ -207,6 +196,10 @@ static bbg_status LaunchTrace(bbg_accel* a, const float4* rays, int64_t n, float
         for (int64_t c = 0; c < n; c += chunk)
         {
             int32_t m = int32_t(std::min(chunk, n - c));
+            // Cleared by every launch, not left clear by the last one: after a
+            // call that overlapped another one (which the contract forbids) the
+            // counter may stand anywhere, and the next call must not inherit it.
+            BBG_CUDA(cudaMemsetAsync(a->work.p, 0, sizeof(int32_t), stream));
             k<<<grid, kTraceBlock, 0, stream>>>(a->view(), rays + 2 * c, m, hits ? hits + c : nullptr,
                                                 occ ? occ + c : nullptr, a->work.p);
         }
@@ -550,8 +543,7 @@ bbg_status CreateAccel(const bbg_geometry* g, const bbg_bvh* bvh, bbg_accel* a, 
         BBG_TRY(copies.Join());
         BBG_TRY(shading.Join());
         BBG_TRY(a->counters.alloc(2));
-        BBG_TRY(a->work.alloc(2));
-        BBG_CUDA(cudaMemsetAsync(a->work.p, 0, 2 * sizeof(int32_t), a->stream));
+        BBG_TRY(a->work.alloc(1));
         BBG_CUDA(cudaStreamSynchronize(a->stream));
         return BBG_OK;
     }
@@ -636,8 +628,7 @@ bbg_status CreateAccel(const bbg_geometry* g, const bbg_bvh* bvh, bbg_accel* a, 
     BBG_TRY(UploadGeometry(a, g));
     BBG_TRY(UploadShading(a, g, a->stream));
     BBG_TRY(a->counters.alloc(2));
-    BBG_TRY(a->work.alloc(2));
-    BBG_CUDA(cudaMemsetAsync(a->work.p, 0, 2 * sizeof(int32_t), a->stream));
+    BBG_TRY(a->work.alloc(1));
     BBG_CUDA(cudaStreamSynchronize(a->stream));
     return BBG_OK;
 }

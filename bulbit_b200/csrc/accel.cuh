@@ -72,7 +72,7 @@ struct bbg_accel
     // Traversal counters (nodes, prims) of the last call when enabled.
     bool counting = false;
     bbg::DevBuf<unsigned long long> counters;
-    bbg::DevBuf<int32_t> work; // persistent kernels: work counter, finished blocks (both 0 between launches)
+    bbg::DevBuf<int32_t> work; // persistent-kernel work counter
     int64_t last_nodes = 0, last_prims = 0;
 
     bbg::AccelView view() const
