@@ -939,8 +939,8 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                     }
                 }
             }
+            __syncwarp(); // the hits have been read that the next round overwrites
         }
-        __syncwarp();
     };
 
     while (true)

@@ -3,6 +3,8 @@ its lanes) against the reference-order traversal, which tests each leaf where
 it meets it: batch sizes around warps and blocks, leaves of one and of many
 primitives, spheres among triangles, intervals of no length, and rays whose
 interval ends at a hit."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -35,6 +37,25 @@ def with_spheres():
     s.prim_kind = np.concatenate([s.prim_kind, np.full(60, abi.BBG_PRIM_SPHERE, np.int32)])
     s.prim_index = np.concatenate([s.prim_index, np.arange(60, dtype=np.int32)])
     s.prim_material = np.full(3060, -1, np.int32)
+    return s
+
+
+def corner_fans(cubes=60):
+    """Per cube, 24 triangles of three of its corners whose box is the whole cube:
+    no split separates them, so a leaf holds them all, at different t."""
+    g = np.random.default_rng(12)
+    corner = np.array([[k & 1, k >> 1 & 1, k >> 2] for k in range(8)], np.float32)
+    tri = [c for c in itertools.combinations(range(8), 3) if np.ptp(corner[list(c)], axis=0).min() == 1][:24]
+    lo, size = g.uniform(-1, 0.7, (cubes, 1, 3)), g.uniform(0.1, 0.3, (cubes, 1, 3))
+    s = scenes.triangle_soup(1, seed=8)
+    s.positions = (lo + corner[None] * size).reshape(-1, 3).astype(np.float32)
+    s.tri_indices = (8 * np.arange(cubes)[:, None, None] + np.array(tri)[None]).reshape(-1, 3).astype(np.int32)
+    s.normals = np.tile(np.float32([0, 1, 0]), (8 * cubes, 1))
+    s.tangents = np.tile(np.float32([1, 0, 0]), (8 * cubes, 1))
+    s.uvs = np.zeros((8 * cubes, 2), np.float32)
+    m = s.tri_indices.shape[0]
+    s.prim_kind, s.prim_index = np.zeros(m, np.int32), np.arange(m, dtype=np.int32)
+    s.prim_material = np.full(m, -1, np.int32)
     return s
 
 
@@ -94,4 +115,24 @@ def test_intervals_around_hits(name):
             assert np.all((got[0] < 0) | (got[1] == rays[:, 6]))
         else:
             check(scene, acc, rays)
+    acc.close()
+
+
+@pytest.mark.parametrize("make", [corner_fans, lambda: stacked(31)], ids=["fans", "stacked31"])
+def test_records_of_large_leaves(make):
+    """32 waiting leaves of two dozen primitives are tested in many rounds: each
+    ray's record (primitive, t, u, v) is one primitive's."""
+    acc = lib.GpuAccel(make())
+    assert acc.export_wide8().shape[0] > 0
+    closest, _ = scenes.soup_rays(100_003, seed=5)
+    acc.set_traversal(abi.BBG_TRAVERSAL_REFERENCE)
+    ref = acc.intersect(closest)
+    acc.set_traversal(abi.BBG_TRAVERSAL_WIDE)
+    got = acc.intersect(closest)
+    assert (ref[0] >= 0).sum() > 5000
+    assert np.array_equal(got[1].view(np.uint32), ref[1].view(np.uint32))
+    # Copies share u and v; two triangles of a fan meet at one t only along the
+    # line they cross in.
+    other = np.any([got[k].view(np.uint32) != ref[k].view(np.uint32) for k in (2, 3)], axis=0)
+    assert np.count_nonzero(other) <= 4
     acc.close()
