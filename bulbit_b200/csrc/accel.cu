@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <cuda.h>
 #include <map>
 #include <mutex>
 #include <thread>
@@ -270,10 +271,54 @@ void KeepHostMesh(bbg_accel* a, const bbg_geometry* g)
     a->host_spheres.assign(g->spheres, g->spheres + size_t(g->n_spheres));
 }
 
+// The calling thread's CUDA state that a thread working on its behalf has to
+// take over: the current context, which may be one of the caller's own instead
+// of the device's primary one (the accel's streams belong to it), and the
+// stream capture mode. The runtime has no call for the former; the driver's is
+// asked of the runtime, so that nothing is linked against the driver.
+class CallerCudaState
+{
+public:
+    // On the calling thread; false: the state cannot be handed on.
+    bool Take()
+    {
+        cudaDriverEntryPointQueryResult found{};
+        void *get = nullptr, *set = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &get, cudaEnableDefault, &found) != cudaSuccess || !get ||
+            cudaGetDriverEntryPoint("cuCtxSetCurrent", &set, cudaEnableDefault, &found) != cudaSuccess || !set)
+        {
+            return false;
+        }
+        set_current_ = reinterpret_cast<CUresult (*)(CUcontext)>(set);
+        if (reinterpret_cast<CUresult (*)(CUcontext*)>(get)(&context_) != CUDA_SUCCESS || !context_)
+        {
+            return false;
+        }
+        mode_ = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&mode_) != cudaSuccess) // mode_: the thread's own
+        {
+            return false;
+        }
+        cudaStreamCaptureMode back = mode_;
+        return cudaThreadExchangeStreamCaptureMode(&back) == cudaSuccess;
+    }
+    // On the other thread.
+    bool Apply() const
+    {
+        cudaStreamCaptureMode mode = mode_;
+        return set_current_(context_) == CUDA_SUCCESS && cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    }
+
+private:
+    CUresult (*set_current_)(CUcontext) = nullptr;
+    CUcontext context_ = nullptr;
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeGlobal;
+};
+
 // A task beside the calling thread's own work; Join (and the destructor)
 // waits for it. An exception in the task becomes its status, and the message
 // of a failed task (messages are per thread) is passed on by Join. Where no
-// thread can be started the task runs in Start.
+// thread can be started, or none in the caller's context, it runs in Start.
 class SideTask
 {
 public:
@@ -284,13 +329,17 @@ public:
             thread_.join();
         }
     }
+    // cuda: the task makes CUDA calls; they run in the caller's context.
     template <class F>
-    void Start(F fn)
+    void Start(F fn, bool cuda)
     {
-        auto body = [this, fn] {
+        CallerCudaState caller;
+        const bool beside = !cuda || caller.Take();
+        auto body = [this, fn, cuda, beside, caller] {
             try
             {
-                status_ = fn();
+                status_ = cuda && beside && !caller.Apply() ? Fail(BBG_ERR_CUDA, "the build's second thread: context")
+                                                            : fn();
             }
             catch (...)
             {
@@ -303,9 +352,15 @@ public:
         };
         try
         {
-            thread_ = std::thread(body);
+            if (beside)
+            {
+                thread_ = std::thread(body);
+            }
         }
         catch (...)
+        {
+        }
+        if (!thread_.joinable())
         {
             body();
         }
@@ -516,14 +571,13 @@ bbg_status CreateAccel(const bbg_geometry* g, const bbg_bvh* bvh, bbg_accel* a, 
         copies.Start([a, g] {
             KeepHostMesh(a, g);
             return BBG_OK;
-        });
+        }, false);
         BBG_TRY(UploadGeometry(a, g));
         shading.Start([a, g] {
-            DeviceScope ds(a->device);
             BBG_TRY(UploadShading(a, g, a->copy_stream[0]));
             BBG_CUDA(cudaStreamSynchronize(a->copy_stream[0]));
             return BBG_OK;
-        });
+        }, true);
         if (device_tree == DeviceTree::SahSplit)
         {
             DevBuf<float4> ref_box;
