@@ -2,6 +2,7 @@
 // tree, and the batched closest-hit / any-hit traversal kernels.
 
 #include "accel.cuh"
+#include "grid_table.h"
 #include "wide8_build.cuh"
 
 #include <algorithm>
@@ -9,10 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cuda.h>
-#include <map>
-#include <mutex>
 #include <thread>
-#include <tuple>
 
 namespace bbg
 {
@@ -49,27 +47,25 @@ int CurrentSmCount()
     return sms;
 }
 
-// Asked of the runtime once per kernel, launch shape and device: a render asks
-// for three dozen of them, a query for one, each some microseconds.
+// A render asks for three dozen grids, a query for one, each some microseconds
+// where the runtime has to answer (see GridTable).
 int PersistentGrid(const void* kernel, int block, size_t smem)
 {
-    static std::mutex mutex;
-    static std::map<std::tuple<const void*, int, size_t, int>, int> grids;
+    static GridTable grids;
     int dev = 0;
     cudaGetDevice(&dev);
-    const std::tuple<const void*, int, size_t, int> key{ kernel, block, smem, dev };
-    std::lock_guard<std::mutex> lock(mutex);
-    auto it = grids.find(key);
-    if (it != grids.end())
+    const GridKey key{ kernel, smem, block, dev };
+    int grid = grids.Find(key);
+    if (grid > 0)
     {
-        return it->second;
+        return grid;
     }
     int per_sm = 1;
     const bool known = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) == cudaSuccess;
-    const int grid = CurrentSmCount() * std::max(per_sm, 1);
+    grid = CurrentSmCount() * std::max(per_sm, 1);
     if (known)
     {
-        grids[key] = grid;
+        grids.Store(key, grid);
     }
     return grid;
 }
