@@ -727,7 +727,9 @@ __device__ __forceinline__ int32_t ChildRef8(const float4* wide8, int32_t node, 
 // group, a group being the hit interior children of one node (node << 8 |
 // visit positions left). A node with hit interior children makes them the
 // current group and pushes what is left of the old one; every push is one
-// tree level deeper than the last, so the tree depth bounds the stack.
+// tree level deeper than the last, so the tree depth bounds the stack. The
+// next node is picked and its reference fetched right after a node's test, so
+// that the fetch runs beside the queueing of the leaves.
 //
 // The primitives of the hit leaves are not tested by the lane that found them
 // but by the whole warp: a hit leaf goes into a queue of the warp in shared
@@ -744,21 +746,35 @@ __device__ __forceinline__ int32_t ChildRef8(const float4* wide8, int32_t node, 
 // left would otherwise fill it too slowly and open nodes behind a hit that it
 // does not know of yet.
 //
+// The nearest hit of each ray stands in shared memory, written by the lane
+// that tested the primitive, and the closest-hit kernels read the origin from
+// there too: both would otherwise be registers that live through the node
+// test, and at 64 registers a single spilled one costs 3 to 5 %.
+//
 // Measured on one B200 against a loop per lane over its own leaves (which ran
-// with 8 to 16 of a warp's 32 threads active, 20 to 23 here): 2^21 incoherent
-// closest-hit rays in the 1,310,734-triangle Cornell box 2.05 -> 1.34 ms, the
-// any-hit rays 1.03 -> 0.67 ms, a 512 x 512, 64-sample frame 151.9 -> 104.2 ms;
-// in the 1,048,576-triangle soup (7 primitives per ray against 28 nodes) 1.60 ->
-// 1.37 ms and 0.33 -> 0.31 ms; 20,000 rays there 228 -> 189 us. Queueing single
+// with 8 to 16 of a warp's 32 threads active, 20 to 23 here), both with the
+// memset of the work counter: 2^21 incoherent closest-hit rays in the
+// 1,310,734-triangle Cornell box 2.05 -> 1.30 ms, the any-hit rays 1.03 -> 0.67
+// ms, a 512 x 512, 64-sample frame 151.9 -> 104.0 ms; in the 1,048,576-triangle
+// soup (7 primitives per ray against 28 nodes) 1.60 -> 1.35 ms and 0.32 -> 0.30
+// ms, 20,000 rays there 161 -> 142 us and 100 -> 96 us; 1,024 rays in a
+// 20,000-triangle soup 79.8 -> 75.8 us; a frame of a 34-triangle box 2.24 -> 2.06
+// ms. Dearer than the loop: small any-hit batches that meet few leaves (20,000
+// small triangles; 300, 1,024 and 20,000 rays 20.8 -> 22.7, 24.4 -> 26.1 and 29.1
+// -> 30.3 us), where a warp has its scheduler to itself and the ballots around
+// the queue lengthen every iteration; in the larger soup the same batches gain
+// (1,024 rays 61.8 -> 57.3 us), so the batch's size does not tell them apart,
+// and emptying the queue sooner, by age or by the share of rays that wait,
+// made them no faster and the large batches 2 to 15 % slower. Queueing single
 // primitives instead of leaves, in a step per primitive, had cost the soup
 // 13 %: the queueing steps were half of all instructions. Without kLeafAge
-// the 20,000 rays took 276 us.
+// 20,000 closest-hit rays in the large soup took 1.45 times as long.
 constexpr int kWarpQueue = 64; // at most 31 waiting leaves + 32 new ones
 constexpr int kWaitFlush = 4;  // 1 to 10 measure alike
 constexpr int kLeafAge = 8;    // 3 to 12 measure alike
 
 template <bool ANY, class Src, int BLOCK = kTraversalBlock, int SHORT = kShortStack, bool SPHERES = true>
-__device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t n, int32_t* next, Src& src)
+__device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t n, int32_t* work, Src& src)
 {
     const unsigned kFull = 0xffffffffu;
     constexpr bool kPerItemView = requires { src.View(0); };
@@ -771,7 +787,7 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
     __shared__ float4 s_org[BLOCK];               // ray origin, t_min
     __shared__ float4 s_dir[BLOCK];               // normalised direction, its length before
     __shared__ float4 s_raw[SPHERES ? BLOCK : 1]; // direction as given (sphere test)
-    __shared__ float4 s_hit[ANY ? 1 : BLOCK];     // hits of a round: primitive, t, u, v
+    __shared__ float4 s_best[ANY ? 1 : BLOCK];    // nearest hit so far: primitive, t, u, v
     __shared__ const float4* s_slots[kPerItemView ? BLOCK : 1];
     __shared__ const float4* s_wide8[kPerItemView ? BLOCK : 1];
     const int warp0 = tid & ~31; // the warp's rays in s_org and s_dir
@@ -789,13 +805,13 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
 
     int32_t item = -1;
     bool exhausted = false;
-    V3 org{}, inv_box{};
-    float t_min = 0, t_max = 0;
-    TraceResult res{ -1, 0, 0, 0 };
+    V3 inv_box{};
+    float t_max = 0;
+    int32_t found = -1; // ANY: 0 once something is hit
     int sp = 0;
     uint32_t oct = 0;
-    uint32_t group = 0;          // current group; kRootGroup: the root is next
-    constexpr uint32_t kRootGroup = 0x80000001u;
+    int32_t next = -1;           // node to open, -1: none left
+    uint32_t group = 0;          // current group, without it
     const float4* wide8 = a.wide8;
     uint32_t lm = 0;             // hit leaves of the node just opened, not queued yet
     uint32_t head = 0, tail = 0; // queue positions: tested, filled (warp-uniform)
@@ -824,6 +840,7 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
         __syncwarp();
         const uint32_t waiting = min(32u, tail - head);
         const uint32_t entry = leaves[(head + lane) & (kWarpQueue - 1)];
+        __syncwarp(); // read before new leaves are written there
         int owner = int(entry >> 26);
         int32_t first = -1, count = 1;
         if (uint32_t(lane) < waiting)
@@ -896,50 +913,73 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                                             &u, &v);
                 }
                 // An interval of no length: only the first primitive counts.
-                hit = hit && (leading || !(ray_t_max <= ro.w));
-            }
-            unsigned hits = __ballot_sync(kFull, hit);
-            if (!ANY && hits != 0)
-            {
-                s_hit[ANY ? 0 : tid] = make_float4(__int_as_float(prim), t, u, v);
-                __syncwarp();
-            }
-            for (; hits != 0; hits &= hits - 1)
-            {
-                const int from = __ffs(hits) - 1;
-                const int to = __shfl_sync(kFull, ray, from);
-                if constexpr (ANY)
+                if (hit && ray_t_max <= ro.w)
                 {
-                    // One hit is enough: the ray is done.
-                    if (lane == to)
-                    {
-                        res.prim = 0;
-                        group = 0;
-                        sp = 0;
-                        lm = 0;
-                    }
+                    hit = leading && (ANY || __float_as_int(s_best[ANY ? 0 : warp0 + ray].x) < 0);
                 }
-                else
+            }
+            if constexpr (ANY)
+            {
+                // One hit is enough: the ray is done.
+                if ((__reduce_or_sync(kFull, hit ? 1u << ray : 0u) >> lane) & 1u)
                 {
-                    // The rule of a loop over the ray's own leaves: nothing
-                    // farther than the nearest hit, and nothing more once that
-                    // is at t_min.
-                    const float ht = __shfl_sync(kFull, t, from);
-                    if (lane == to && !(ht > t_max) && (res.prim < 0 || !(t_max <= t_min)))
+                    found = 0;
+                    next = -1;
+                    sp = 0;
+                    lm = 0;
+                }
+            }
+            else
+            {
+                // The hits' lanes write the records, all at once where no ray
+                // has two (handing them over one by one instead cost closed
+                // scenes, where most lanes hit, 5 to 10 %), else in the order of
+                // the queue by the rule of a loop over the ray's own leaves:
+                // nothing farther than the nearest hit (the primitive's test
+                // has seen to that for a ray's first), and nothing more once
+                // that is at t_min.
+                const unsigned hits = __ballot_sync(kFull, hit);
+                if (hits != 0)
+                {
+                    const unsigned rays = __reduce_or_sync(kFull, hit ? 1u << ray : 0u);
+                    const float4 record = make_float4(__int_as_float(prim), t, u, v);
+                    if (__popc(rays) == __popc(hits))
                     {
-                        const float4 h = s_hit[ANY ? 0 : warp0 + from];
-                        res = TraceResult{ __float_as_int(h.x), ht, h.z, h.w };
-                        t_max = ht;
-                        if (t_max <= t_min)
+                        if (hit)
                         {
-                            group = 0;
+                            s_best[ANY ? 0 : warp0 + ray] = record;
+                        }
+                    }
+                    else
+                    {
+                        for (unsigned left = hits; left != 0; left &= left - 1)
+                        {
+                            if (lane == __ffs(left) - 1)
+                            {
+                                const float4 best = s_best[ANY ? 0 : warp0 + ray];
+                                if (!(t > best.y) &&
+                                    (__float_as_int(best.x) < 0 || !(best.y <= s_org[warp0 + ray].w)))
+                                {
+                                    s_best[ANY ? 0 : warp0 + ray] = record;
+                                }
+                            }
+                            __syncwarp();
+                        }
+                    }
+                    __syncwarp();
+                    if ((rays >> lane) & 1u)
+                    {
+                        t_max = s_best[ANY ? 0 : tid].y;
+                        if (t_max <= s_org[tid].w)
+                        {
+                            next = -1;
                             sp = 0;
                             lm = 0;
                         }
                     }
+                    __syncwarp(); // read before the next round writes there
                 }
             }
-            __syncwarp(); // the hits have been read that the next round overwrites
         }
     };
 
@@ -954,7 +994,7 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
             int32_t base = 0;
             if (lane == 0)
             {
-                base = atomicAdd(next, cnt);
+                base = atomicAdd(work, cnt);
             }
             base = __shfl_sync(kFull, base, 0);
             exhausted = base + cnt >= n;
@@ -965,8 +1005,8 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                 {
                     item = r;
                     RayQ q;
+                    float t_min;
                     src.Load(r, &q, &t_min, &t_max);
-                    org = q.o;
                     inv_box = q.inv_box;
                     s_org[tid] = make_float4(q.o.x, q.o.y, q.o.z, t_min);
                     s_dir[tid] = make_float4(q.dn.x, q.dn.y, q.dn.z, q.l);
@@ -981,10 +1021,15 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                         s_wide8[tid] = av.wide8;
                         s_slots[tid] = av.slots;
                     }
-                    res = TraceResult{ -1, t_max, 0, 0 };
+                    found = -1;
+                    if (!ANY)
+                    {
+                        s_best[ANY ? 0 : tid] = make_float4(__int_as_float(-1), t_max, 0.0f, 0.0f);
+                    }
                     sp = 0;
                     oct = uint32_t(inv_box.x < 0) | (uint32_t(inv_box.y < 0) << 1) | (uint32_t(inv_box.z < 0) << 2);
-                    group = kRootGroup;
+                    next = 0; // the root
+                    group = 0;
                     last = head;
                 }
             }
@@ -995,21 +1040,12 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
             break;
         }
         uint32_t entry = 0;
-        if ((group & 0xffu) != 0 || sp > 0)
+        if (next >= 0)
         {
-            if ((group & 0xffu) == 0)
-            {
-                group = pop();
-            }
-            const uint32_t pos = uint32_t(__ffs(group) - 1);
-            int32_t node = 0; // the root
-            if (group != kRootGroup)
-            {
-                node = ChildRef8(wide8, int32_t(group >> 8), pos ^ oct);
-            }
-            group &= group - 1;
+            const int32_t node = next;
             uint32_t im;
-            IntersectNode8(wide8 + 6 * size_t(node), org, inv_box, t_min, t_max,
+            const float4 ro = s_org[tid];
+            IntersectNode8(wide8 + 6 * size_t(node), V3{ ro.x, ro.y, ro.z }, inv_box, ro.w, t_max,
                            reinterpret_cast<const uint8_t*>(s_order) + (oct << 8), &im, &lm);
             if (im != 0)
             {
@@ -1018,6 +1054,17 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                     push(group);
                 }
                 group = (uint32_t(node) << 8) | im;
+            }
+            // The next node: its reference is under way while the leaves queue.
+            if ((group & 0xffu) == 0 && sp > 0)
+            {
+                group = pop();
+            }
+            next = -1;
+            if ((group & 0xffu) != 0)
+            {
+                next = ChildRef8(wide8, int32_t(group >> 8), uint32_t(__ffs(group) - 1) ^ oct);
+                group &= group - 1;
             }
             entry = (uint32_t(lane) << 26) | (uint32_t(node) << 3);
         }
@@ -1033,10 +1080,10 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                 last = tail + uint32_t(__popc(adding & below));
                 leaves[last & (kWarpQueue - 1)] = entry | (pos ^ oct);
                 ++last;
-                if (t_max <= t_min)
+                if (t_max <= s_org[tid].w)
                 {
                     // An interval of no length: the first leaf is the last one.
-                    group = 0;
+                    next = -1;
                     sp = 0;
                     lm = 0;
                 }
@@ -1046,7 +1093,7 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
             if (adding == 0 && head != tail)
             {
                 // Lanes with no node left wait for their leaves.
-                const bool walking = (group & 0xffu) != 0 || sp > 0;
+                const bool walking = next >= 0;
                 const unsigned walk = __ballot_sync(kFull, walking);
                 const unsigned wait = __ballot_sync(kFull, !walking && item >= 0 && int32_t(last - head) > 0);
                 flush = walk == 0 || __popc(wait) >= kWaitFlush || ++age >= kLeafAge;
@@ -1061,11 +1108,11 @@ __device__ __forceinline__ void TracePersistentWide(const AccelView& a, int32_t 
                 break;
             }
         }
-        if (item >= 0 && (group & 0xffu) == 0 && sp == 0 && int32_t(last - head) <= 0)
+        if (item >= 0 && next < 0 && int32_t(last - head) <= 0)
         {
-            src.Store(item, res);
+            const float4 b = ANY ? make_float4(__int_as_float(found), t_max, 0.0f, 0.0f) : s_best[ANY ? 0 : tid];
+            src.Store(item, TraceResult{ __float_as_int(b.x), b.y, b.z, b.w });
             item = -1;
-            group = 0;
         }
     }
 }
