@@ -666,7 +666,6 @@ bbg_status CreateAccel(const bbg_geometry* g, const bbg_bvh* bvh, bbg_accel* a, 
         if (BuildWide8(a->host_nodes, &wide8, &a->depth8))
         {
             a->n_wide8 = int32_t(wide8.size() / 6);
-            a->root8 = 0;
             a->use_wide8 = true; // the default traversal where the layout exists
             BBG_TRY(a->wide8.upload(wide8.data(), wide8.size(), a->stream));
         }

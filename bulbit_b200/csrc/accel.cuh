@@ -24,7 +24,6 @@ struct bbg_accel
     int32_t root = 0;
     bool ordered = true;
     bbg::DevBuf<float4> wide8; // 6 float4 per node (8-wide layout; empty if not built)
-    int32_t root8 = 0;
     int32_t n_wide8 = 0;
     int32_t depth8 = 0;
     bool use_wide8 = false;    // ordered queries run over the 8-wide layout
@@ -77,7 +76,7 @@ struct bbg_accel
 
     bbg::AccelView view() const
     {
-        return bbg::AccelView{ nodes.p, slots.p, wide.p, leaves.p, root, ordered ? 1 : 0, wide8.p, root8 };
+        return bbg::AccelView{ nodes.p, slots.p, wide.p, leaves.p, root, ordered ? 1 : 0, wide8.p };
     }
     bool wide8_active() const { return ordered && use_wide8 && wide8.p != nullptr; }
 };

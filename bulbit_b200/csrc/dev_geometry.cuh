@@ -29,8 +29,7 @@ struct AccelView
     const int2* leaves;   // (first slot, count) per leaf
     int32_t root;         // child-box layout root reference
     int32_t ordered;      // 1: nearest-first traversal over the child-box layout
-    const float4* wide8 = nullptr; // 8-wide layout: 6 per node (null: not built)
-    int32_t root8 = 0;             // 8-wide root node
+    const float4* wide8 = nullptr; // 8-wide layout: 6 per node, the root first (null: not built)
 };
 
 struct RayQ

@@ -391,7 +391,6 @@ static bbg_status BuildWide8OnDevice(bbg_accel* a, int32_t n, const DevBuf<int2>
         end = state[0];
     }
     a->n_wide8 = end;
-    a->root8 = 0;
     a->depth8 = depth;
     a->use_wide8 = true;
     return BBG_OK;

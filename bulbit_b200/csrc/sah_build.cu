@@ -1336,7 +1336,6 @@ bbg_status SahWide8(bbg_accel* a, const bbg_bvh_node* nd, int32_t n_nodes, int s
         end += state[0];
     }
     a->n_wide8 = end;
-    a->root8 = 0;
     a->depth8 = depth;
     a->use_wide8 = true;
     return BBG_OK;
