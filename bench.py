@@ -1004,12 +1004,13 @@ def main():
                    "parallelism": f"replicas x{world}", "bvh_build_s": round(build_s, 3)},
         # The tree and triangles stay in L2 (DRAM traffic is ~2 % of the
         # algorithmic bytes), so the kernel is bound by instruction issue:
-        # achieved / frac are the algorithmic bytes per launch over its time
-        # against the HBM copy peak (the byte-equivalent rate the reference's
-        # traversal work would need), issue_active / alu_pipe_active the
-        # measured issue and ALU utilisation (ncu, profiles/).
-        "roofline": {"bound": "issue", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                     "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
+        # achieved / frac are the share of the issue slots that it uses (ncu
+        # capture of the same kernel, profiles/). reference_work_gbs is the
+        # reference traversal's algorithmic bytes per launch over its time, a
+        # byte-equivalent rate and no use of the HBM.
+        "roofline": {"bound": "issue", "achieved": prof.get("issue_active"), "peak": 1.0,
+                     "unit": "warp instructions per scheduler and cycle", "frac": prof.get("issue_active"),
+                     "traffic": traffic, "reference_work_gbs": achieved, "hbm_peak_gbs": peaks["hbm_gbs"],
                      "issue_active": prof.get("issue_active"), "alu_pipe_active": prof.get("alu_pipe_active"),
                      "threads_per_instruction": prof.get("threads_per_instruction"),
                      "profile": "profiles/trace_closest_soup1m.md",

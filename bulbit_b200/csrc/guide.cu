@@ -1231,7 +1231,8 @@ bbg_status GuideAccumulate(bbg_guide* G, const float* raw_dev, const float* dirs
     // One CTA per (chunk, layer); chunks past the batch exit at once.
     GuideWeightGradTcKernel<<<dim3(unsigned(chunks), 4), kTcThreads, kTcSmem, st>>>(G->scratch.p, ld, n_dev, n_host,
                                                                                      G->partial.p, G->tc_status.p);
-    GuideGradReduceKernel<<<kWeightEntries / kReduceWeights, kReduceWeights * kReduceParts, 0, st>>>(G->partial.p, n_dev, n_host, G->grad.p);
+    GuideGradReduceKernel<<<kWeightEntries / kReduceWeights, kReduceWeights * kReduceParts, 0, st>>>(
+        G->partial.p, n_dev, n_host, G->grad.p);
     BBG_CUDA(cudaGetLastError());
     return BBG_OK;
 }
